@@ -779,10 +779,12 @@ __device__ bool band_factor_forward(const TopoInst& I, const double* __restrict_
   };
   // chunk ch: warp w stages column gj = jlo + ch TD_JC + w, its lanes the rows
   // (L(K + r, gj) sits at Lb[gj ld + K - gj + r] while r <= rmax = bw - K + gj).
-  // The products read a column's rows only up to rmax + 10 (the row blocks a
-  // 4-column step needs) and the last row block (right-hand side, row R), so
-  // only rows < rmax + 17 and that block are staged (zero beyond the band);
-  // columns past the panel start (gj >= K) are staged as zeros throughout.
+  // The products read rows 0 .. TD_NB - 1 of every column (the panel's own columns,
+  // times the right-hand-side row in all of them), its rows up to rmax + 10 (the row
+  // blocks a 4-column step needs) and the last row block (right-hand side, row R):
+  // rows < max(rmax + 17, TD_NB) and that block are staged, zero beyond the band, and
+  // so is all of a column past the panel start (gj >= K).  What is not staged is
+  // another chunk's, or whatever ran on the SM before.
   auto issue = [&](int K, int ch) {
     const int jlo = max(0, K - bw), nch = (K - jlo + TD_JC - 1) / TD_JC;
     if (ch < nch) {
@@ -791,7 +793,7 @@ __device__ bool band_factor_forward(const TopoInst& I, const double* __restrict_
       const bool live = gj < K;
       const double* col = Lb + (int64_t)gj * ld + (K - gj);
       const int rmax = live ? bw - (K - gj) : -1;
-      const int rz = live ? min(rmax + 17, rlast) : rlast;  // (pairs of rows)
+      const int rz = live ? min(max(rmax + 17, TD_NB), rlast) : rlast;  // (pairs of rows)
       for (int r = 2 * lane; r < rz; r += 64) td_cp16(Wj + r, r <= rmax ? col + r : Lb, rmax + 1 - r);
       if (lane < 8) td_cp8(Wj + rlast + lane, live && rlast + lane == R ? yb + gj : Lb, live && rlast + lane == R);
     }
