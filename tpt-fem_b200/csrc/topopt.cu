@@ -1512,8 +1512,8 @@ void topopt_batch(tptfem_context* ctx, const tptfem_topopt_instance* in, int n, 
   DevBuf<uint8_t> dfixed;
   d_inst.alloc(n, s); d_order.alloc(n, s); d_last.alloc(n, s); d_flags.alloc(n, s); d_total.alloc(n, s);
   d_ok.alloc(n, s); d_refine.alloc(n, s); d_dorder.alloc(std::max(ndirect, 1), s);
-  dL.alloc(loff + 64 * (TD_MAXBW + 2), s);  // (loads ahead may pass an instance's end)
-  dyb.alloc(yoff + 1024, s);
+  dL.alloc(std::max<int64_t>(loff, 1), s);
+  dyb.alloc(std::max<int64_t>(yoff, 1), s);
   for (auto* v : {&ex, &ephys, &eE, &eraw, &esens, &exnew}) v->alloc(std::max<int64_t>(eoff, 1), s);
   for (auto* v : {&df, &dlift, &dfix, &du, &dr, &dp, &dq, &ddinv, &db}) v->alloc(std::max<int64_t>(doff, 1), s);
   dfixed.alloc(std::max<int64_t>(doff, 1), s);
@@ -1527,13 +1527,6 @@ void topopt_batch(tptfem_context* ctx, const tptfem_topopt_instance* in, int n, 
   dfix.upload(ufix.data(), doff);
   dfixed.upload(fixed.data(), doff);
   if (ndirect) d_dorder.upload(dorder.data(), ndirect);
-  // The band storage's entries past a column's band and the vectors' first values are
-  // read before they are written, against zero factors or as a first guess: zero, so
-  // that what the pool held before (a NaN) has no part (2 ms for the 8.6 GB of 512
-  // instances, once per call)
-  dL.zero();
-  dyb.zero();
-  for (auto* v : {&ex, &ephys, &eE, &eraw, &esens, &exnew, &du, &dr, &dp, &dq, &ddinv, &db}) v->zero();
   d_last.zero(); d_flags.zero(); d_total.zero(); dhist.zero(); d_ok.zero(); d_refine.zero();
 
   TopoArgs a{};
