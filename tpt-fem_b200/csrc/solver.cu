@@ -102,6 +102,7 @@ struct Engine {
   const T* va = nullptr;
   Precond<T> pc;
   DevBuf<T> xl, r, p, q, z, t, dinv;
+  int dinv_gen = -1;  // generation of the values that dinv was taken from
   DevBuf<double> partials;
   DevBuf<PcgState> st;
   cudaGraphExec_t exec = nullptr;
@@ -414,26 +415,24 @@ void flag_check(tptfem_context* ctx, const char* msg) {
   TPT_REQUIRE(ctx->h_pinned[0] == 0, TPTFEM_ERR_NUMERIC, msg);
 }
 
-template <typename T>
-void prepare_jacobi(SystemData& S, Engine<T>& E, const T* va, int batch) {
-  cudaStream_t s = S.ctx->stream;
-  E.setup((int)S.n_free, S.row_ptr.p, S.col.p, va, S.nnz, s, batch);
-  TPT_CUDA(cudaMemsetAsync(S.ctx->d_flag, 0, sizeof(int), s));
-  jacobi_diag<T><<<ceil_div(S.n_free, 256), 256, 0, s>>>((int)S.n_free, S.row_ptr.p, S.col.p, S.val.p, E.dinv.p,
-                                                         S.ctx->d_flag);
-  TPT_CHECK_LAUNCH();
-  flag_check(S.ctx, "reduced matrix has a missing or non-positive diagonal entry (not SPD)");
-  E.pc.kind = PC_JACOBI;
-}
-
+// 1 / diagonal of the present values (throws if one is not positive).
 template <typename T>
 void refresh_jacobi(SystemData& S, Engine<T>& E) {
   cudaStream_t s = S.ctx->stream;
+  E.dinv_gen = -1;
   TPT_CUDA(cudaMemsetAsync(S.ctx->d_flag, 0, sizeof(int), s));
   jacobi_diag<T><<<ceil_div(S.n_free, 256), 256, 0, s>>>((int)S.n_free, S.row_ptr.p, S.col.p, S.val.p, E.dinv.p,
                                                          S.ctx->d_flag);
   TPT_CHECK_LAUNCH();
   flag_check(S.ctx, "reduced matrix has a missing or non-positive diagonal entry (not SPD)");
+  E.dinv_gen = S.value_gen;
+}
+
+template <typename T>
+void prepare_jacobi(SystemData& S, Engine<T>& E, const T* va, int batch) {
+  E.setup((int)S.n_free, S.row_ptr.p, S.col.p, va, S.nnz, S.ctx->stream, batch);
+  refresh_jacobi(S, E);
+  E.pc.kind = PC_JACOBI;
 }
 
 // ||b - A x||^2 in FP64 into W.rhi / returned.
@@ -767,12 +766,6 @@ void system_solve(SystemData& S, const tptfem_solver_opts& o_in, tptfem_solve_st
         nb_fill_factor(S, W.fsai);
         W.nb_factor = &W.fsai;
       }
-    } else if (solver == TPTFEM_SOLVER_JACOBI_PCG && (o.flags & TPTFEM_SOLVE_CSR_ONLY) && W.f64_csr_ready) {
-      refresh_jacobi<double>(S, W.f64_csr);
-    } else if (solver == TPTFEM_SOLVER_JACOBI_PCG && !(o.flags & TPTFEM_SOLVE_CSR_ONLY) && W.f64_ready) {
-      refresh_jacobi<double>(S, W.f64);
-    } else if (solver == TPTFEM_SOLVER_MP_PCG && W.f32_ready) {
-      refresh_jacobi<float>(S, W.f32);
     }
   }
   if (solver == TPTFEM_SOLVER_FSAI_MP_PCG) {
@@ -795,18 +788,30 @@ void system_solve(SystemData& S, const tptfem_solver_opts& o_in, tptfem_solve_st
     }
   }
   const bool csr_only = (o.flags & TPTFEM_SOLVE_CSR_ONLY) != 0;
-  if (solver == TPTFEM_SOLVER_JACOBI_PCG && csr_only && !W.f64_csr_ready) {
-    prepare_jacobi<double>(S, W.f64_csr, S.val.p, batch);
+  // an engine that was last used for other values takes its preconditioner from the
+  // present ones, whatever solved the system in between
+  auto stale = [&](const auto& E) { return (o.flags & TPTFEM_SOLVE_FRESH_SETUP) || E.dinv_gen != S.value_gen; };
+  if (solver == TPTFEM_SOLVER_JACOBI_PCG && csr_only) {
+    if (!W.f64_csr_ready) prepare_jacobi<double>(S, W.f64_csr, S.val.p, batch);
+    else if (stale(W.f64_csr)) refresh_jacobi<double>(S, W.f64_csr);
     W.f64_csr_ready = true;
   }
-  if (solver == TPTFEM_SOLVER_JACOBI_PCG && !csr_only && !W.f64_ready) {
-    prepare_jacobi<double>(S, W.f64, S.val.p, batch);
-    if (nb_build_operator(S)) W.f64.use_nb(&S.nb, true, false);
+  if (solver == TPTFEM_SOLVER_JACOBI_PCG && !csr_only) {
+    if (!W.f64_ready) {
+      prepare_jacobi<double>(S, W.f64, S.val.p, batch);
+      if (nb_build_operator(S)) W.f64.use_nb(&S.nb, true, false);
+    } else if (stale(W.f64)) {
+      refresh_jacobi<double>(S, W.f64);
+    }
     W.f64_ready = true;
   }
-  if (solver == TPTFEM_SOLVER_MP_PCG && !W.f32_ready) {
-    ensure_val32(S);
-    prepare_jacobi<float>(S, W.f32, S.val32.p, batch);
+  if (solver == TPTFEM_SOLVER_MP_PCG) {
+    if (!W.f32_ready) {
+      ensure_val32(S);
+      prepare_jacobi<float>(S, W.f32, S.val32.p, batch);
+    } else if (stale(W.f32)) {
+      refresh_jacobi<float>(S, W.f32);
+    }
     W.f32_ready = true;
   }
   st.solver_used = solver;
