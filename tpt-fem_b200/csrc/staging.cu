@@ -3,13 +3,14 @@
 // The C ABI takes ordinary (pageable) host arrays.  Large ones are copied by
 // several host threads into the context's pinned staging buffer (kept between
 // calls, grown on demand) in chunks, each moved by its own DMA as soon as it is
-// filled (downloads the same way in reverse), instead of the driver's
-// single-threaded pageable path; connectivity is narrowed to int32 and
+// filled (downloads the same way in reverse, through a few chunks of it), instead
+// of the driver's single-threaded pageable path; connectivity is narrowed to int32 and
 // coefficients are checked on the way.  Small arrays go directly.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -20,13 +21,21 @@ namespace tptfem {
 namespace {
 
 constexpr size_t STAGE_MIN_BYTES = 1u << 20;  // below this the direct copy is as fast
-constexpr size_t STAGE_CHUNK = 8u << 20;      // pipelined transfers move chunks of this size
+constexpr size_t STAGE_CHUNK = 8u << 20;      // uploads move chunks of this size
+// Downloads: chunks of this size, and how many of them are in flight.  First to_csr of
+// a context and later ones, 3.8M entries: one slot for every chunk (55 MB and more)
+// 20-27 and 5.4 ms, 4 x 4 MB 16-20 and 2.7, 3 x 4 MB 12 and 2.9, 4 x 2 MB 9-11 and 3.2;
+// 99.8M entries: 530-1000 and 58 ms (1.2 GB of pinned memory), 70-80 and 54, 70 and 55,
+// 70-80 and 63.  Pageable copies: 22 and 18, 570 and 484.
+constexpr size_t STAGE_OUT_CHUNK = 4u << 20;
+constexpr size_t STAGE_RING = 3;
 
 unsigned stage_threads(size_t bytes) {
   const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
   return (unsigned)std::max<size_t>(1, std::min<size_t>(std::min(16u, hw), bytes / (1u << 18)));
 }
 
+// The pinned buffer, of at least `bytes`.
 void* stage(tptfem_context* ctx, size_t bytes) {
   if (ctx->h_stage_bytes < bytes) {
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
@@ -36,6 +45,17 @@ void* stage(tptfem_context* ctx, size_t bytes) {
     ctx->h_stage_bytes = bytes;
   }
   return ctx->h_stage;
+}
+
+// The same, null where there is none to be had.
+void* try_stage(tptfem_context* ctx, size_t bytes) {
+  try {
+    return stage(ctx, bytes);
+  } catch (const Error&) {
+    ctx->h_stage = nullptr;  // (what a failed call leaves is not defined)
+    cudaGetLastError();
+    return nullptr;
+  }
 }
 
 // Host -> device through the pinned buffer, pipelined: n staged elements of
@@ -98,27 +118,35 @@ void host_to_device(tptfem_context* ctx, void* dst, const void* src, size_t byte
   });
 }
 
-// Device -> host through the pinned buffer, pipelined: chunk c's DMA is
-// followed by an event; host thread t copies its slice of each chunk out once
-// that chunk's event has completed (int32 indices widened to int64 on the way),
-// while the next chunks are still moving.  All arrays of a call share one
-// pipeline and one team of threads: the three arrays of a 4.6M-entry matrix
-// 18.7 -> 3.2 ms against pageable copies and a widening loop.
+// Device -> host through the pinned buffer, pipelined: chunk k's DMA is followed by
+// an event; host thread t copies its slice of each chunk out once that chunk's event
+// has completed (int32 indices widened to int64 on the way), while the next chunks
+// are still moving.  The chunks go round a ring of STAGE_RING slots, so the pinned
+// memory stays small whatever is downloaded: chunk k is issued when every thread has
+// copied chunk k - STAGE_RING out.  All arrays of a call share one pipeline and one
+// team of threads.  Small arrays, and all where no pinned memory is to be had, go as
+// pageable copies with a widening loop.
 void device_to_host(tptfem_context* ctx, const HostCopy* copies, int ncopies) {
   struct Chunk {
     const HostCopy* c;
-    size_t first, count, at;  // elements of the array, bytes into the staging buffer
+    size_t first, count;  // elements of the array
   };
-  size_t bytes = 0;
+  size_t bytes = 0, slot = 0;  // of all arrays, of a ring slot
   std::vector<Chunk> chunks;
   for (int k = 0; k < ncopies; ++k) {
     const HostCopy& c = copies[k];
-    const size_t cel = STAGE_CHUNK / c.elem;
-    for (size_t i = 0; i < c.count; i += cel) chunks.push_back({&c, i, std::min(cel, c.count - i), bytes + i * c.elem});
-    bytes += (c.count * c.elem + 255) & ~(size_t)255;
+    const size_t cel = STAGE_OUT_CHUNK / c.elem;
+    for (size_t i = 0; i < c.count; i += cel) {
+      chunks.push_back({&c, i, std::min(cel, c.count - i)});
+      slot = std::max(slot, chunks.back().count * c.elem);
+    }
+    bytes += c.count * c.elem;
   }
   if (!bytes) return;
-  if (bytes < STAGE_MIN_BYTES) {
+  slot = (slot + 255) & ~(size_t)255;
+  const size_t n = chunks.size(), ring = std::min(n, STAGE_RING);
+  char* p = bytes < STAGE_MIN_BYTES ? nullptr : static_cast<char*>(try_stage(ctx, ring * slot));
+  if (!p) {
     std::vector<int> narrow;
     for (int k = 0; k < ncopies; ++k) {
       const HostCopy& c = copies[k];
@@ -131,44 +159,76 @@ void device_to_host(tptfem_context* ctx, const HostCopy* copies, int ncopies) {
     }
     return;
   }
-  char* p = static_cast<char*>(stage(ctx, bytes));
-  std::vector<cudaEvent_t> ev(chunks.size(), nullptr);
-  cudaError_t issued = cudaSuccess;
-  for (size_t k = 0; k < chunks.size() && issued == cudaSuccess; ++k) {
+  const unsigned nt = stage_threads(bytes);
+  std::vector<cudaEvent_t> ev(ring, nullptr);
+  std::vector<std::atomic<unsigned>> out(n);  // slices of a chunk that have been copied out
+  for (auto& o : out) o.store(0);
+  std::atomic<size_t> issued(0);
+  std::atomic<bool> failed(false);
+  cudaError_t err = cudaSuccess;
+  auto issue = [&](size_t k) {
     const Chunk& c = chunks[k];
-    issued = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming);
-    if (issued == cudaSuccess)
-      issued = cudaMemcpyAsync(p + c.at, static_cast<const char*>(c.c->src) + c.first * c.c->elem, c.count * c.c->elem,
-                               cudaMemcpyDeviceToHost, ctx->stream);
-    if (issued == cudaSuccess) issued = cudaEventRecord(ev[k], ctx->stream);
-  }
-  std::atomic<int> err(0);
-  if (issued == cudaSuccess) {
-    const unsigned nt = stage_threads(bytes);
-    auto work = [&](unsigned t) {
-      for (size_t k = 0; k < chunks.size(); ++k) {
-        if (cudaEventSynchronize(ev[k]) != cudaSuccess) { err = 1; return; }
-        const Chunk& c = chunks[k];
-        const size_t b = c.count * t / nt, e = c.count * (t + 1) / nt;
-        if (c.c->widen) {
-          const int* from = reinterpret_cast<const int*>(p + c.at);
-          int64_t* to = static_cast<int64_t*>(c.c->dst) + c.first;
-          for (size_t i = b; i < e; ++i) to[i] = from[i];
-        } else {
-          std::memcpy(static_cast<char*>(c.c->dst) + (c.first + b) * c.c->elem, p + c.at + b * c.c->elem,
-                      (e - b) * c.c->elem);
-        }
+    cudaEvent_t& e = ev[k % ring];
+    if (!e) err = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+    if (err == cudaSuccess)
+      err = cudaMemcpyAsync(p + k % ring * slot, static_cast<const char*>(c.c->src) + c.first * c.c->elem,
+                            c.count * c.c->elem, cudaMemcpyDeviceToHost, ctx->stream);
+    if (err == cudaSuccess) err = cudaEventRecord(e, ctx->stream);
+    if (err == cudaSuccess) issued.store(k + 1, std::memory_order_release);
+    else failed = true;
+  };
+  auto copy_out = [&](size_t k, unsigned t) {
+    const Chunk& c = chunks[k];
+    const char* from = p + k % ring * slot;
+    const size_t b = c.count * t / nt, e = c.count * (t + 1) / nt;
+    if (c.c->widen) {
+      const int* v = reinterpret_cast<const int*>(from);
+      int64_t* to = static_cast<int64_t*>(c.c->dst) + c.first;
+      for (size_t i = b; i < e; ++i) to[i] = v[i];
+    } else {
+      std::memcpy(static_cast<char*>(c.c->dst) + (c.first + b) * c.c->elem, from + b * c.c->elem, (e - b) * c.c->elem);
+    }
+    out[k].fetch_add(1, std::memory_order_release);
+  };
+  auto work = [&](unsigned t) {
+    for (size_t k = 0; k < n; ++k) {
+      while (issued.load(std::memory_order_acquire) <= k) {
+        if (failed) return;
+        std::this_thread::yield();
       }
-    };
-    std::vector<std::thread> th;
+      if (cudaEventSynchronize(ev[k % ring]) != cudaSuccess) { failed = true; return; }
+      copy_out(k, t);
+    }
+  };
+  std::vector<std::thread> th;
+  th.reserve(nt);
+  try {
     for (unsigned t = 1; t < nt; ++t) th.emplace_back(work, t);
-    work(0);
-    for (auto& x : th) x.join();
+  } catch (const std::system_error&) {  // no more threads: this one copies the slices that are left
   }
+  const unsigned alone = 1 + (unsigned)th.size();
+  size_t next = 0;
+  for (size_t k = 0; k < n && !failed; ++k) {
+    // every chunk whose slot is free goes out; chunk k itself is waited for
+    while (next < n && next < k + ring && !failed) {
+      if (next >= ring && out[next - ring].load(std::memory_order_acquire) < nt) {
+        if (next > k) break;
+        std::this_thread::yield();
+        continue;
+      }
+      issue(next++);
+    }
+    if (failed) break;
+    if (cudaEventSynchronize(ev[k % ring]) != cudaSuccess) { failed = true; break; }
+    copy_out(k, 0);
+    for (unsigned t = alone; t < nt; ++t) copy_out(k, t);
+  }
+  for (auto& x : th) x.join();
+  if (failed) cudaStreamSynchronize(ctx->stream);  // nothing moves into the buffer any more
   for (auto e : ev)
     if (e) cudaEventDestroy(e);
-  TPT_CUDA(issued);
-  TPT_REQUIRE(!err, TPTFEM_ERR_DEVICE, "device-to-host copy failed");
+  TPT_CUDA(err);
+  TPT_REQUIRE(!failed, TPTFEM_ERR_DEVICE, "device-to-host copy failed");
 }
 
 void device_to_host(tptfem_context* ctx, void* dst, const void* src, size_t bytes) {
