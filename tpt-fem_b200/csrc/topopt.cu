@@ -32,6 +32,7 @@
 
 #include "common.cuh"
 #include "objects.hpp"
+#include "pivot_rcp.cuh"
 
 namespace tptfem {
 namespace {
@@ -553,17 +554,6 @@ __device__ __forceinline__ void td_mma(double& d0, double& d1, double a, double 
                : "d"(a), "d"(b));
 }
 
-// 1 / x by Newton-Raphson from the hardware's approximate reciprocal
-// (rcp.approx.ftz.f64, PTX ISA: relative error below 2^-20): two steps square it
-// to below double rounding.  x: pivots; a subnormal one gives no finite result
-// and the factorisation counts as broken down.
-__device__ __forceinline__ double td_rcp(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  r = r * (2.0 - x * r);
-  return r * (2.0 - x * r);
-}
-
 __device__ __forceinline__ int band_index(const TopoInst& I, int i, int j, int comp) {
   return 2 * (I.yfast ? i * I.ny + j : j * I.nx + i) + comp;
 }
@@ -752,8 +742,8 @@ __device__ __forceinline__ void td_rank4(double* p, const double (&f)[4], const 
   }
 }
 
-// Factor K_FF = L L^T into Lb and solve L y = yb in place.  False on a
-// non-positive pivot.
+// Factor K_FF = L L^T into Lb and solve L y = yb in place.  False on a pivot that is
+// not positive or has no reciprocal here.
 template <int NT, int NSTAGE>
 __device__ bool band_factor_forward(const TopoInst& I, const double* __restrict__ E, const uint8_t* __restrict__ fixed,
                                     const double* __restrict__ ke, double* Lb, double* yb, double* sm, int* bad) {
@@ -878,7 +868,6 @@ __device__ bool band_factor_forward(const TopoInst& I, const double* __restrict_
         c0[j] = Pa[j * PS + lane];
         c1[j] = Pa[(4 + j) * PS + lane];
       }
-      bool okp = true;
 #pragma unroll 1
       for (int g = 0; g < TD_NB / 4; ++g) {
         double* cg = colb + 4 * g * TD_NB;
@@ -892,7 +881,6 @@ __device__ bool band_factor_forward(const TopoInst& I, const double* __restrict_
             myd = d;
             dinv[lane] = iv;
           }
-          okp = okp && d > 0.0 && isfinite(d);
           f[i] = c0[i] * iv;
 #pragma unroll
           for (int j = i + 1; j < 4; ++j) c0[j] -= f[i] * __shfl_sync(0xffffffffu, c0[i], 4 * g + j);
@@ -916,7 +904,7 @@ __device__ bool band_factor_forward(const TopoInst& I, const double* __restrict_
         }
       }
       rsq[lane] = rsqrt(myd);
-      if (!okp && lane == 0) *bad = 1;
+      if (!(myd >= TD_PIVOT_MIN && myd <= TD_PIVOT_MAX)) *bad = 1;
       __syncwarp();
       td_bar_arrive(TD_NB / 4 + 1, 32 * nwp);
     } else if (warp < nwp) {
