@@ -256,16 +256,6 @@ struct RnArgs {
   int max_it;
 };
 
-template <int DPN>
-size_t rn_smem(int nc, int w, int na, int nseg) {
-  const size_t rows = (size_t)nc * 32 * DPN;
-  const int nm = rigid_modes(DPN);
-  return (6 * rows + (size_t)nc * w * DPN * 32) * sizeof(double) +
-         (na ? (((size_t)na + nseg) * nm + RP_THREADS * nm) * sizeof(double) +
-                   ((size_t)na * 2 + nseg + (size_t)nc * 32) * sizeof(int)
-             : 0);
-}
-
 template <int DPN, bool FSAI>
 __global__ void __launch_bounds__(RP_THREADS, 1) resident_nb(RnArgs A) {
   constexpr int D2 = DPN * DPN, NM = rigid_modes(DPN), CR = 32 * DPN;
@@ -776,6 +766,11 @@ const void* rn_kernel(bool fsai) {
   return fsai ? (const void*)resident_nb<DPN, true> : (const void*)resident_nb<DPN, false>;
 }
 
+RnShape shape_of(const SystemData& S, bool coarse) {
+  const CoarseSpace& C = S.coarse;
+  return rn_shape(S.nb.nchunks, S.nb.dpn, sm_count(), coarse ? C.na : 0, coarse ? C.nm : 0, coarse ? C.nseg : 0);
+}
+
 RpOutcome outcome(const SystemData& S, const RpResult* d_res) {
   cudaStream_t s = S.ctx->stream;
   RpResult h{};
@@ -801,8 +796,9 @@ bool resident_jacobi_applies(const SystemData& S) {
 
 bool resident_nb_applies(const SystemData& S, bool fsai, bool coarse) {
   const NbSell& N = S.nb;
-  return N.state == 1 && S.n_free > 0 && S.n_free <= (fsai ? RN_MAX_ROWS_FSAI : RN_MAX_ROWS_JACOBI) &&
-         (!coarse || (S.coarse.nc <= RN_MAX_COARSE && S.coarse.nseg <= RN_MAX_SEG));
+  if (N.state != 1 || S.n_free <= 0 || S.n_free > (fsai ? RN_MAX_ROWS_FSAI : RN_MAX_ROWS_JACOBI)) return false;
+  if (coarse && (S.coarse.nc > RN_MAX_COARSE || S.coarse.nseg > RN_MAX_SEG)) return false;
+  return shape_of(S, coarse).smem <= RN_MAX_SMEM;  // (a part of a GPU has fewer SMs for the same rows)
 }
 
 RpOutcome resident_jacobi_solve(SystemData& S, ResidentWork& W, double tol, double delta, int64_t max_it) {
@@ -836,9 +832,10 @@ RpOutcome resident_nb_solve(SystemData& S, ResidentWork& W, const float* sigma2,
   RnArgs A{};
   A.ngroups = N.ngroups;
   A.nchunks = N.nchunks;
-  A.nc = ceil_div(N.nchunks, std::min(sm_count(), RP_MAX_BLOCKS));
-  const int blocks = ceil_div(N.nchunks, A.nc);
-  A.w = A.nc == 1 ? 16 : A.nc == 2 ? 8 : A.nc <= 4 ? 4 : A.nc <= 8 ? 2 : 1;
+  const RnShape shape = shape_of(S, coarse);
+  const int blocks = shape.blocks;
+  A.nc = shape.nc;
+  A.w = shape.w;
   A.lcptr = N.l_cptr.p; A.lcol = N.l_col.p; A.ucptr = N.u_cptr.p; A.ucol = N.u_col.p; A.ubase = N.ku_base.p;
   A.lval = N.ks_lval.p; A.dval = N.ks_diag.p;
   A.lpack = N.l_pack.p; A.upack = N.u_pack.p; A.ltail = N.l_tail.p; A.utail = N.u_tail.p; A.ldiag = N.l_diag.p;
@@ -873,12 +870,9 @@ RpOutcome resident_nb_solve(SystemData& S, ResidentWork& W, const float* sigma2,
   A.delta = delta;
   A.max_it = (int)std::min<int64_t>(max_it, 1 << 30);
   const void* k = N.dpn == 3 ? rn_kernel<3>(fsai) : N.dpn == 2 ? rn_kernel<2>(fsai) : rn_kernel<1>(fsai);
-  const size_t smem = N.dpn == 3   ? rn_smem<3>(A.nc, A.w, A.na, A.nseg)
-                      : N.dpn == 2 ? rn_smem<2>(A.nc, A.w, A.na, A.nseg)
-                                   : rn_smem<1>(A.nc, A.w, A.na, A.nseg);
-  TPT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TPT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shape.smem));
   void* args[] = {&A};
-  TPT_CUDA(cudaLaunchCooperativeKernel(k, dim3(blocks), dim3(RP_THREADS), args, smem, s));
+  TPT_CUDA(cudaLaunchCooperativeKernel(k, dim3(blocks), dim3(RP_THREADS), args, shape.smem, s));
   return outcome(S, A.res);
 }
 

@@ -10,11 +10,10 @@
 // whatever order stores arrive, and waits for the values it needs only.
 #pragma once
 #include "common.cuh"
+#include "resident_shape.hpp"
 
 namespace tptfem {
 
-constexpr int RP_THREADS = 512;
-constexpr int RP_MAX_BLOCKS = 160;  // a multiple of 32
 // Repeats of one load before a kernel gives up (about a second): the launch is
 // cooperative, so every block is resident and a wait ends in microseconds.
 constexpr int RP_POLL_LIMIT = 1 << 21;
