@@ -1379,6 +1379,8 @@ void launch_nodes_tet(int mode, const RowArgs& A, int64_t n_nodes, cudaStream_t 
   TPT_CHECK_LAUNCH();
 }
 
+constexpr size_t AR_MAX_SMEM = 227 * 1024;
+
 template <int CELL, int PHYS, int DPN>
 void launch_rows(int mode, const RowArgs& A, cudaStream_t s) {
   // Threads per block: the dense accumulator (9 bytes per slot and thread)
@@ -1386,9 +1388,9 @@ void launch_rows(int mode, const RowArgs& A, cudaStream_t s) {
   int threads = 128;
   while (threads > 32 && (size_t)threads * A.maxc * 9 > 200 * 1024) threads -= 32;
   size_t smem = (size_t)threads * A.maxc * 9;
-  TPT_REQUIRE(smem <= 227 * 1024, TPTFEM_ERR_CREATION, "node valence too high for the device assembly path");
+  TPT_REQUIRE(smem <= AR_MAX_SMEM, TPTFEM_ERR_CREATION, "node valence too high for the device assembly path");
   auto run = [&](auto kern) {
-    TPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem((const void*)kern, AR_MAX_SMEM);
     kern<<<ceil_div(A.nrows, threads), threads, smem, s>>>(A);
     TPT_CHECK_LAUNCH();
   };

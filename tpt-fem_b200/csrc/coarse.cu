@@ -748,10 +748,9 @@ bool coarse_build(SystemData& S, int target) {
     }
   }
   C.T.alloc(T.size(), s); C.T.upload(T.data(), T.size());
-  TPT_CUDA(cudaFuncSetAttribute(cs_gemv, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(CS_MAX_COARSE * sizeof(double))));
-  TPT_CUDA(cudaFuncSetAttribute(dpn == 3 ? cs_solve<6> : dpn == 2 ? cs_solve<3> : cs_solve<1>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(CS_MAX_COARSE * sizeof(double))));
+  allow_smem((const void*)cs_gemv, CS_MAX_COARSE * sizeof(double));
+  allow_smem(dpn == 3 ? (const void*)cs_solve<6> : dpn == 2 ? (const void*)cs_solve<3> : (const void*)cs_solve<1>,
+             CS_MAX_COARSE * sizeof(double));
   C.Ac.alloc((size_t)C.nc * C.nc, s);
   C.info.alloc(1, s);  // on the context's stream, which outlives the engines' second streams
   C.ld = (C.nc + 3) & ~3;

@@ -75,6 +75,13 @@ struct DevBuf {
   }
 };
 
+// Lets launches of a kernel use up to `most` bytes of dynamic shared memory.  The limit
+// is the process's, so it is the same on every call: one set to what the next launch
+// needs is another thread's before that launch.
+inline void allow_smem(const void* kernel, size_t most) {
+  TPT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+}
+
 inline int ceil_div(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
 // Error-free transformations (Knuth TwoSum; TwoProduct through FMA), for the

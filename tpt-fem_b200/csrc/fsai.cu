@@ -492,7 +492,7 @@ void launch_fsai_nodes(const SystemData& S, FsaiFactor& F, double* sig2, double*
   }
   auto run = [&](auto kernel, size_t per_warp, int per_sm, const int* rows) {
     const size_t bytes = 4 * per_warp;
-    TPT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    allow_smem((const void*)kernel, bytes);  // (one size per kernel)
     kernel<<<std::min(ceil_div(n, 4), per_sm * sm_count()), 128, bytes, s>>>(
         S.dpn, S.free_map.p, S.row_ptr.p, S.col.p, S.val.p, F.rp.p, F.ci.p, sig2, lva, S.ctx->d_flag, rows);
     TPT_CHECK_LAUNCH();

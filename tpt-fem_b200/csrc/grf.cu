@@ -53,7 +53,7 @@ void grf_eval(tptfem_context* ctx, const double* h_points, int64_t n, const doub
   d_pts.alloc(3 * chunk, s);
   d_out.alloc(chunk, s);
   const size_t shmem = 4 * (size_t)M * sizeof(double);
-  TPT_CUDA(cudaFuncSetAttribute(grf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem));
+  allow_smem((const void*)grf_kernel, 4 * (size_t)GRF_MAX_FEATURES * sizeof(double));
   for (int64_t p0 = 0; p0 < n; p0 += chunk) {
     const int64_t len = std::min(chunk, n - p0);
     host_to_device(ctx, d_pts.p, h_points + 3 * p0, 3 * len * sizeof(double));

@@ -46,6 +46,7 @@ constexpr int RN_WARPS = RP_THREADS / 32;
 // LANES lanes share a row of the CSR matrix (L1-resident), the vectors lie in
 // shared memory: an iteration is three block barriers.
 constexpr int RJ_THREADS = 512;
+constexpr size_t RJ_MAX_SMEM = 6 * (RJ_MAX_LANES / 4) * sizeof(double);  // four lanes a row at least
 
 struct RjArgs {
   int n;
@@ -818,7 +819,7 @@ RpOutcome resident_jacobi_solve(SystemData& S, ResidentWork& W, double tol, doub
   const int lanes = rj_lanes(S.n_free, S.nnz);
   auto* k = lanes == 4 ? resident_jacobi<4> : lanes == 8 ? resident_jacobi<8> : resident_jacobi<16>;
   const size_t smem = 6 * (size_t)A.n * sizeof(double);
-  TPT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem((const void*)k, RJ_MAX_SMEM);
   k<<<1, RJ_THREADS, smem, s>>>(A);
   TPT_CHECK_LAUNCH();
   return outcome(S, A.res);
@@ -870,7 +871,7 @@ RpOutcome resident_nb_solve(SystemData& S, ResidentWork& W, const float* sigma2,
   A.delta = delta;
   A.max_it = (int)std::min<int64_t>(max_it, 1 << 30);
   const void* k = N.dpn == 3 ? rn_kernel<3>(fsai) : N.dpn == 2 ? rn_kernel<2>(fsai) : rn_kernel<1>(fsai);
-  TPT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shape.smem));
+  allow_smem(k, RN_MAX_SMEM);
   void* args[] = {&A};
   TPT_CUDA(cudaLaunchCooperativeKernel(k, dim3(blocks), dim3(RP_THREADS), args, shape.smem, s));
   return outcome(S, A.res);

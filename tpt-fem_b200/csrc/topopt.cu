@@ -505,20 +505,26 @@ static_assert(TD_NT == 16 * TD_NB, "backward dot products use 16 lanes per panel
 
 // column stride of the band storage: bw + 1 entries and one of padding, so that an
 // even row of any column (bw is odd) starts on a 16-byte boundary
-__host__ __device__ inline int td_ld(int bw) { return bw + 2; }
+__host__ __device__ constexpr int td_ld(int bw) { return bw + 2; }
 // rows stored per panel: R = bw + TD_NB matrix rows, the right-hand-side row R, padding to 4
-__host__ __device__ inline int td_rs(int bw) { return (bw + TD_NB + 1 + 7) & ~7; }
+__host__ __device__ constexpr int td_rs(int bw) { return (bw + TD_NB + 1 + 7) & ~7; }
 // column stride of the panels and chunks in shared memory: 8 modulo 16 doubles, so
 // that the tiles' accesses (4 columns x 8 rows) take the fewest bank passes
-__host__ __device__ inline int td_cs(int rs) { return rs | 8; }
+__host__ __device__ constexpr int td_cs(int rs) { return rs | 8; }
 // two panels, the chunk buffers and the published columns
-__host__ __device__ inline int64_t td_smem_doubles(int bw, int stages) {
+__host__ __device__ constexpr int64_t td_smem_doubles(int bw, int stages) {
   const int cs = td_cs(td_rs(bw));
   return 2LL * TD_NB * (cs + 4) + (int64_t)stages * TD_JC * cs + TD_NB * TD_NB;
 }
 // chunk buffers: four while they fit beside the panels
 constexpr int64_t TD_SMEM_MAX = 224 * 1024 / sizeof(double);
-__host__ __device__ inline int td_stages(int bw) { return td_smem_doubles(bw, 4) <= TD_SMEM_MAX ? 4 : 2; }
+__host__ __device__ constexpr int td_stages(int bw) { return td_smem_doubles(bw, 4) <= TD_SMEM_MAX ? 4 : 2; }
+// dynamic shared memory of the widest band
+constexpr size_t td_most_smem() {
+  int64_t most = 0;
+  for (int bw = 1; bw <= TD_MAXBW; ++bw) most = std::max(most, td_smem_doubles(bw, td_stages(bw)));
+  return (size_t)most * sizeof(double);
+}
 static_assert(((TD_MAXBW + TD_NB + 1 + 7) & ~7) <= TD_RSMAX, "TD_MAXBW must fit TD_RSMAX");
 constexpr int TD_RING = 512;  // unknowns kept by the backward substitution: a window of R and a panel
 static_assert(TD_RING >= TD_RSMAX + TD_NB, "the window must fit the ring");
@@ -1489,8 +1495,7 @@ void topopt_batch(tptfem_context* ctx, const tptfem_topopt_instance* in, int n, 
   const int stages = td_stages(max_bw);
   const auto direct_kernel = stages == 4 ? topo_direct<TD_NT, 4> : topo_direct<TD_NT, 2>;
   const int64_t td_smem = td_smem_doubles(max_bw, stages) * (int64_t)sizeof(double);
-  if (ndirect)
-    TPT_CUDA(cudaFuncSetAttribute(direct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)td_smem));
+  if (ndirect) allow_smem((const void*)direct_kernel, td_most_smem());
 
   DevBuf<TopoInst> d_inst;
   DevBuf<int> d_order, d_last, d_flags, d_dorder, d_ok;
