@@ -21,13 +21,12 @@ namespace tptfem {
 namespace {
 
 constexpr size_t STAGE_MIN_BYTES = 1u << 20;  // below this the direct copy is as fast
-constexpr size_t STAGE_CHUNK = 8u << 20;      // uploads move chunks of this size
-// Downloads: chunks of this size, and how many of them are in flight.  First to_csr of
-// a context and later ones, 3.8M entries: one slot for every chunk (55 MB and more)
-// 20-27 and 5.4 ms, 4 x 4 MB 16-20 and 2.7, 3 x 4 MB 12 and 2.9, 4 x 2 MB 9-11 and 3.2;
-// 99.8M entries: 530-1000 and 58 ms (1.2 GB of pinned memory), 70-80 and 54, 70 and 55,
-// 70-80 and 63.  Pageable copies: 22 and 18, 570 and 484.
-constexpr size_t STAGE_OUT_CHUNK = 4u << 20;
+constexpr size_t STAGE_CHUNK = 8u << 20;      // pipelined transfers move chunks of this size
+// Chunks of a download in flight.  to_csr with 3.8M entries (46 MB), the first of a
+// context and later ones: a slot for every chunk 20-27 and 2.4 ms, three slots 17-20 and
+// 2.5 (of 4 MB 12 and 2.7, of 2 MB 8 and 3.6: the threads' slices get short), pageable
+// copies 22 and 18.  With 99.8M entries: 530-1000 and 58 ms (1.2 GB of pinned memory),
+// 80-110 and 54, 570 and 484.
 constexpr size_t STAGE_RING = 3;
 
 unsigned stage_threads(size_t bytes) {
@@ -135,7 +134,7 @@ void device_to_host(tptfem_context* ctx, const HostCopy* copies, int ncopies) {
   std::vector<Chunk> chunks;
   for (int k = 0; k < ncopies; ++k) {
     const HostCopy& c = copies[k];
-    const size_t cel = STAGE_OUT_CHUNK / c.elem;
+    const size_t cel = STAGE_CHUNK / c.elem;
     for (size_t i = 0; i < c.count; i += cel) {
       chunks.push_back({&c, i, std::min(cel, c.count - i)});
       slot = std::max(slot, chunks.back().count * c.elem);
@@ -200,6 +199,8 @@ void device_to_host(tptfem_context* ctx, const HostCopy* copies, int ncopies) {
       copy_out(k, t);
     }
   };
+  size_t next = 0;
+  while (next < ring && !failed) issue(next++);  // (before there are threads that wait on events)
   std::vector<std::thread> th;
   th.reserve(nt);
   try {
@@ -207,11 +208,10 @@ void device_to_host(tptfem_context* ctx, const HostCopy* copies, int ncopies) {
   } catch (const std::system_error&) {  // no more threads: this one copies the slices that are left
   }
   const unsigned alone = 1 + (unsigned)th.size();
-  size_t next = 0;
   for (size_t k = 0; k < n && !failed; ++k) {
     // every chunk whose slot is free goes out; chunk k itself is waited for
     while (next < n && next < k + ring && !failed) {
-      if (next >= ring && out[next - ring].load(std::memory_order_acquire) < nt) {
+      if (out[next - ring].load(std::memory_order_acquire) < nt) {
         if (next > k) break;
         std::this_thread::yield();
         continue;
