@@ -111,7 +111,10 @@ typedef struct tptfem_solver_opts {
 /* Node-block operator: use the full block storage of K instead of the default
  * symmetric half storage (lower blocks + diagonal, the upper half applied as
  * the transposes of the lower blocks; K is symmetric up to the FP64 rounding
- * of its element matrices, and the FP64 true residual always uses K itself). */
+ * of its element matrices, and the FP64 true residual always uses K itself).
+ * It also keeps the solve of a small system to separate kernels: by default that is
+ * one cooperative launch, which begins when all its SMs are free at once, so not
+ * before a kernel of another stream that holds one ends. */
 #define TPTFEM_SOLVE_FULL_OPERATOR 4
 /* FSAI / learned-FSAI solvers: add an aggregation coarse correction,
  * M^-1 = G^T G + P A_c^-1 P^T, with P the rigid-body modes (translations and

@@ -28,6 +28,11 @@
 // breakdown (solves past FP64's accuracy otherwise ended in one).  With
 // two sums: 9,840 rows 5.1 us, 104,544 rows 10.9, FSAI at 14,520 rows 14.3; the same
 // iterations to the solution.
+//
+// A cooperative grid begins when all its SMs are free at once.  Beside another stream's
+// ordinary kernels that costs little (103,823 rows beside 8192^3 GEMMs: 2.8 ms a solve,
+// 38 with the engine's kernels), but a kernel that holds an SM for seconds holds up a
+// solve of as many blocks as there are SMs; TPTFEM_SOLVE_FULL_OPERATOR selects the engine.
 #include <algorithm>
 #include <cmath>
 
@@ -547,8 +552,9 @@ __global__ void __launch_bounds__(RP_THREADS, 1) resident_nb(RnArgs A) {
   bool fresh = true, started = false;  // r is a true residual, not the recurrence's
   bool direct = false;                 // z holds the direction itself (below)
   int done = 0;
-  // (one copy of the preconditioner, of K z and of the sums: the loop body has to
-  // stay in registers and in the instruction cache)
+  // (one copy of the preconditioner, of K z and of the sums: the loop body has to stay
+  // in the instruction cache and, but for 180 bytes that FSAI with 3 dofs reloads and 24
+  // with 2, in registers)
   for (;;) {
     if (FSAI && !direct) {
       __syncthreads();
@@ -757,6 +763,10 @@ __global__ void __launch_bounds__(RP_THREADS, 1) resident_nb(RnArgs A) {
   if (blockIdx.x == 0 && t == 0) *A.res = out;
 }
 
+// Lanes per row of the one-block solve, so that a row's entries take few passes.
+// Microseconds an iteration with 4 / 8 / 16: 125 rows of 5.8 entries 2.8 / 2.9 / 3.9, 343 of
+// 6.1 3.3 / 4.3; 81 rows of 20.8 2.1 / 2.4 / 2.7, 264 of 16.0 2.9 / 3.7, so up to 23 entries
+// four lanes would do (rows of more than 24 have not been measured).
 int rj_lanes(int64_t n, int64_t nnz) {
   const double avg = (double)nnz / (double)std::max<int64_t>(n, 1);
   return avg <= 12 ? 4 : avg <= 40 ? 8 : 16;

@@ -13,10 +13,17 @@ constexpr size_t RN_MAX_SMEM = 226 * 1024;
 struct RnShape {
   int nc;      // chunks of 32 node groups per block
   int blocks;  // one per SM at most: they wait for one another
-  int w;       // warps per chunk, a power of two: 16 warps over the chunks that a block has
+  int w;       // warps per chunk, a power of two (below)
   size_t smem;
 };
 
+// Warps per chunk: the block's 16 over its chunks, rounded down to a power of two.
+// Microseconds an iteration with 1 / 2 / 4 / 8 / 16 of them (the choice in brackets):
+// 2 chunks (9,840 rows, Jacobi) 5.0 / 4.1 / 3.7 / [3.8] / 4.6, (14,520, FSAI) 23.4 / 16.7 /
+// 13.7 / [13.1] / 15.4; 3 chunks (37,800, FSAI) 26.9 / 19.5 / [16.0] / 17.8 / 21.0; 8 chunks
+// (105,840, FSAI) 35.0 / [27.1] / 28.3 / 32.0 / 43.0; 14 chunks (187,500, Jacobi) [14.3] /
+// 15.0 / 15.9 / 16.0 / 19.8; 22 chunks (103,823, Jacobi) [7.5] / 7.7 / 8.9 / 12.8 / 21.3.
+//
 // na, nm, nseg: aggregates, modes and segments of the coarse space (na 0: none).
 inline RnShape rn_shape(int nchunks, int dpn, int sms, int na, int nm, int nseg) {
   const int most = sms < RP_MAX_BLOCKS ? sms : RP_MAX_BLOCKS;

@@ -336,8 +336,10 @@ void ensure_work(SystemData& S) {
 // Node-block engines use the symmetric half storage of K unless the caller
 // asks for the full operator (TPTFEM_SOLVE_FULL_OPERATOR), or the system has one
 // dof per node: there the half storage's second index per upper slot is as large
-// as the value it saves (128^3 Poisson: full 204 MB in 39 us, half 172 MB in 50).
-// The resident solves read the half storage.
+// as the value it saves.  An iteration of the classic two-level Poisson solve, half
+// and full: 157,464 rows 40.2 and 39.2 us, 250,047 46.2 and 42.9, 493,039 60.9 and
+// 61.3, 857,375 107 and 99, 2,048,383 200 and 172 (the operator alone 50 and 39).
+// The resident solves, which end at RN_MAX_ROWS_FSAI rows, read the half storage.
 bool nb_wants_sym(const SystemData& S, const tptfem_solver_opts& o) {
   if (o.flags & TPTFEM_SOLVE_FULL_OPERATOR) return false;
   return S.nb.dpn > 1 || S.n_free <= RN_MAX_ROWS_FSAI;
