@@ -47,6 +47,11 @@ namespace {
 
 constexpr int RN_WARPS = RP_THREADS / 32;
 
+// b as the true residual of x = 0: an infinite entry is a NaN there (inf - inf in the
+// compensated sum), which ends the solve as a breakdown, where the sums of squares would
+// take infinity for converged.
+__device__ __forceinline__ double residual_of_zero(double b) { return b + (b - b); }
+
 // ---- Jacobi-PCG of a system that one block holds ----------------------------------------
 // LANES lanes share a row of the CSR matrix (L1-resident), the vectors lie in
 // shared memory: an iteration is three block barriers.
@@ -107,7 +112,7 @@ __global__ void __launch_bounds__(RJ_THREADS, 1) resident_jacobi(RjArgs A) {
     for (int k = A.rp[i]; k < A.rp[i + 1]; ++k)
       if (__ldg(A.ci + k) == i) d = __ldg(A.va + k);
     if (!(d > 0.0)) v[2] += 1.0;
-    const double di = 1.0 / d, bi = A.b[i];
+    const double di = 1.0 / d, bi = residual_of_zero(A.b[i]);
     dinv[i] = di;
     r[i] = bi;
     p[i] = di * bi;
@@ -532,7 +537,7 @@ __global__ void __launch_bounds__(RP_THREADS, 1) resident_nb(RnArgs A) {
     xl[i] = p[i] = kp[i] = r[i] = z[i] = e[i] = 0.0;  // (padding rows stay zero)
     if (!row_of(i, gl, a)) continue;
     const int64_t row = (int64_t)(g0 + gl) * DPN + a;
-    const double bi = A.b[row];
+    const double bi = residual_of_zero(A.b[row]);
     if (!FSAI) {
       const double d = A.dval[((int64_t)(c0 + i / CR) * D2 + a * DPN + a) * 32 + lane];
       if (!(d > 0.0)) bad += 1.0;
